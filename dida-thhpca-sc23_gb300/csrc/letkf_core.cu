@@ -479,7 +479,8 @@ cudaError_t launch_overlap(letkf_ctx *ctx, const LgGrid &g, const double *xb, co
     if (e != cudaSuccess) return e;
     const int *list = nullptr;
     const unsigned long long *nlist = nullptr;
-    if (K <= 64 && lg_f64_supports(K) && (e = lg_launch_overlap_f64(ctx, g, xb, axb, xa, axa, list, nlist)) != cudaSuccess)
+    if (K <= 64 && lg_f64_supports(K) && lg_aligned16(xb) && lg_aligned16(xa) &&
+        (e = lg_launch_overlap_f64(ctx, g, xb, axb, xa, axa, list, nlist)) != cudaSuccess)
         return e;
     const int64_t ncol = (int64_t)g.nlat * g.nlon;
     const unsigned blocks = list ? 512u : (unsigned)(ncol < (1 << 30) ? ncol : (1 << 30));
@@ -553,8 +554,10 @@ cudaError_t lg_launch_core_fp64(letkf_ctx *ctx, const LgGrid &g, const double *x
     double *tr = keep_trans ? ctx->d_trans.p : nullptr, *w = keep_trans ? ctx->d_w.p : nullptr;
     // the FP64 pipe does two multiply-adds per clock and SM; the whole run, k =
     // 64, 16,200 columns: 308 ms with k_core_fp64, 15.5 on the tensor cores; k = 32:
-    // 60.1 and 6.8; k = 96, 8,978 columns: 736 and 29.4
-    if (lg_f64_supports(g.k) && !ctx->members_on) {
+    // 60.1 and 6.8; k = 96, 8,978 columns: 736 and 29.4.  Its update moves 16
+    // bytes at a time: a caller's device arrays that start between those
+    // boundaries stay with k_core_fp64
+    if (lg_f64_supports(g.k) && !ctx->members_on && lg_aligned16(xb) && lg_aligned16(xa)) {
         bool done = false;
         const cudaError_t e = lg_launch_core_f64(ctx, g, src, ctx->cur_nobs, ctx->d_loff.p, ctx->d_lcnt.p, ctx->win0,
                                                  ctx->win1, xb, axb, xa, axa, tr, w, done);

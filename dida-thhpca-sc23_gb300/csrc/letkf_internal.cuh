@@ -539,9 +539,11 @@ cudaError_t lg_launch_core_fp64(letkf_ctx *ctx, const LgGrid &g, const double *x
 cudaError_t lg_launch_core_mixed(letkf_ctx *ctx, const LgGrid &g, const double *xb,
                                  const double *axb, double *xa, double *axa, bool keep_trans);
 // The FP64 form on the tensor cores (letkf_f64.cu) for the problems of cubes
-// cube0 .. cube1 - 1 (k of lg_f64_supports; rows: rows of the source's y);
+// cube0 .. cube1 - 1 (k of lg_f64_supports; rows: rows of the source's y; xb and
+// xa on 16-byte boundaries);
 // done = false when its intermediates do not fit the device's free memory.
 bool lg_f64_supports(int k);
+inline bool lg_aligned16(const void *p) { return ((uintptr_t)p & 15) == 0; }
 cudaError_t lg_launch_core_f64(letkf_ctx *ctx, const LgGrid &g, const LgRowSrc &src, int64_t rows,
                                const int64_t *loff, const int32_t *lcnt, int64_t cube0, int64_t cube1,
                                const double *xb, const double *axb, double *xa, double *axa, double *trans_out,
