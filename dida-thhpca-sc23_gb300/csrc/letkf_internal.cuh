@@ -151,7 +151,7 @@ struct LgParams {
     int cube_step;        // grid points between cube starts (cube_n - overlap)
     int64_t cube0;        // first cube of the launch's window
     int count_only;       // search: only each cube's list length (LgListMeta::need)
-    uint32_t spin_limit;  // polls of each bounded mbarrier wait of the mixed cores
+    uint32_t spin_limit;  // polls of each bounded mbarrier wait of the tensor-core kernels
     // The caller's conversion around the analysis fused into it
     // (letkf_gpu_run_members, run_da_parallel in module_da_parallel.F90:
     // 163-261): the state input is the full members and there is no mean

@@ -298,12 +298,13 @@ int letkf_gpu_set_list_limit(letkf_ctx *ctx, int64_t max_entries);
  * windows and the work-queue schedule leave every result unchanged.          */
 int letkf_gpu_set_cube_range(letkf_ctx *ctx, int64_t first, int64_t count);
 
-/* Most polls of each bounded wait of the mixed cores on their own
- * tensor-core work (polls < 0: the default, 2^22; 0: every wait gives up at
- * once).  A wait that runs out makes the run return LETKF_ERR_TIMEOUT after
- * the kernel has let its committed products finish and freed its tensor
- * memory, so the context stays usable.  For tests of that path; no
- * counterpart in the reference.                                             */
+/* Most polls of each bounded wait of the tensor-core kernels (the mixed cores,
+ * and the FP64 form's at ensembles of 32, 48, 64, 96 and 128) on their own
+ * work (polls < 0: the default, 2^22; 0: every wait gives up at once).  A wait
+ * that runs out makes the run return LETKF_ERR_TIMEOUT after the kernel has
+ * let its committed products finish and freed its tensor memory, so the
+ * context stays usable.  For tests of that path; no counterpart in the
+ * reference.                                                                */
 int letkf_gpu_set_wait_limit(letkf_ctx *ctx, int64_t polls);
 
 /* Keep (1) or drop (0) every cube's trans and w of the following runs in
