@@ -1336,6 +1336,8 @@ int letkf_gpu_core_batch(letkf_ctx *ctx, int64_t nb, const int64_t *offsets, con
     ctx->have_run = false;
     if (e != cudaSuccess) return set_err(ctx, LETKF_ERR_CUDA, cudaGetErrorString(e));
     if (rc) return rc;
+    if (st & LG_ST_TIMEOUT)
+        return set_err(ctx, LETKF_ERR_TIMEOUT, "a bounded wait on the tensor cores ran out");
     if (st & LG_ST_NOT_CONV)
         return set_err(ctx, LETKF_ERR_NOT_CONVERGED, "an eigensolve reached its sweep limit");
     return LETKF_OK;

@@ -35,3 +35,21 @@ def test_timeout_leaves_context_usable(letkf, k, kw):
         ctx.set_wait_limit(-1)
         xa, axa = ctx.run(w.xb, w.axb, w.obs)
         assert np.array_equal(xa, xa_ref) and np.array_equal(axa, axa_ref)
+
+
+@pytest.mark.parametrize("k", [32, 64, 96])
+def test_core_batch_reports_the_timeout(letkf, k):
+    g = np.random.default_rng(k)
+    off = np.array([0, 0, 150, 350], dtype=np.int64)
+    t = int(off[-1])
+    prob = (off, g.standard_normal((t, k)), np.ones(t, np.float32), g.standard_normal(t), g.uniform(0.1, 1.0, t))
+    glat, glon = pkg("synthetic").make_grid(30.0)
+    ctx = letkf.LetkfGPU(glat, glon, 1, k, loc_dist_km=500.0, inflation=1.1)
+    tr0, w0 = ctx.core_batch(*prob)
+    ctx.set_wait_limit(0)
+    with pytest.raises(letkf.LetkfError) as ei:
+        ctx.core_batch(*prob)
+    assert ei.value.code == letkf.LETKF_ERR_TIMEOUT
+    ctx.set_wait_limit(-1)
+    tr, w = ctx.core_batch(*prob)
+    assert np.array_equal(tr, tr0) and np.array_equal(w, w0)
