@@ -1310,9 +1310,7 @@ int letkf_gpu_core_batch(letkf_ctx *ctx, int64_t nb, const int64_t *offsets, con
     int rc = reset_status(ctx);
     if (rc) return rc;
     LG_CUDA(h2d(ctx->d_boff, offsets, (size_t)nb, ctx->stream));
-    LG_CUDA(ctx->d_lcnt.reserve((size_t)std::max<int64_t>(nb, ctx->ncubes)));
-    LG_CUDA(cudaMemcpyAsync(ctx->d_lcnt.p, cnt.data(), sizeof(int32_t) * nb, cudaMemcpyHostToDevice,
-                            ctx->stream));
+    LG_CUDA(h2d(ctx->d_bcnt, cnt.data(), (size_t)nb, ctx->stream));
     LG_CUDA(h2d(ctx->d_bhx, hxens, (size_t)std::max<int64_t>(total, 1) * k * (total > 0), ctx->stream));
     LG_CUDA(h2d(ctx->d_brdi, rdiaginv, (size_t)total, ctx->stream));
     LG_CUDA(h2d(ctx->d_bdep, dep, (size_t)total, ctx->stream));
@@ -1332,7 +1330,7 @@ int letkf_gpu_core_batch(letkf_ctx *ctx, int64_t nb, const int64_t *offsets, con
     cudaStreamSynchronize(ctx->stream);
     dt.release();
     dw.release();
-    // the per-cube counts of the last run were overwritten
+    // the status and the counters of the last run were overwritten
     ctx->have_run = false;
     if (e != cudaSuccess) return set_err(ctx, LETKF_ERR_CUDA, cudaGetErrorString(e));
     if (rc) return rc;

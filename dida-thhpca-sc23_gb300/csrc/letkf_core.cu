@@ -606,11 +606,11 @@ cudaError_t lg_launch_core_batch_fp64(letkf_ctx *ctx, int64_t nb, int64_t rows, 
     LgGrid g = lg_grid(ctx);
     if (lg_f64_supports(g.k)) {
         bool done = false;
-        const cudaError_t e = lg_launch_core_f64(ctx, g, src, rows, d_off, ctx->d_lcnt.p, 0, nb, nullptr, nullptr,
+        const cudaError_t e = lg_launch_core_f64(ctx, g, src, rows, d_off, ctx->d_bcnt.p, 0, nb, nullptr, nullptr,
                                                  nullptr, nullptr, d_trans, d_w, done);
         if (e != cudaSuccess || done) return e;
     }
-    return dispatch(ctx, g, src, d_off, ctx->d_lcnt.p, 0, nb, nullptr, nullptr, nullptr, nullptr,
+    return dispatch(ctx, g, src, d_off, ctx->d_bcnt.p, 0, nb, nullptr, nullptr, nullptr, nullptr,
                     d_trans, d_w);
 }
 

@@ -32,6 +32,7 @@ struct LgF64Block {
     float *amax;               // largest diagonal element of A'
     int *flag, *list;          // 1: solved by k_core_fp64; the flagged problems
     unsigned long long *cnt;   // F64_CNT_N counters
+    const float *rowmax;       // largest |element| of every row of y
 };
 
 namespace {

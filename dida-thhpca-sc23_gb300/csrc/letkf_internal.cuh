@@ -302,6 +302,19 @@ class LgCopyAgent {
     std::thread thread_;
 };
 
+// Buffers of the FP64 form's tensor-core path (letkf_f64.cu), one set for a
+// block of problems: A or T' as integers, A in FP32, eigenvectors and
+// eigenvalues, the largest diagonal element of A', g or u, flags and list of the
+// problems left to k_core_fp64 and the exponents of A, counters, row maxima of
+// y; k = 96, 128: scratch of each CTA.
+struct LgF64Scratch {
+    DevBuf<long long> A, cta;
+    DevBuf<float> A32, X, lam, amax, rowmax;
+    DevBuf<double> g;
+    DevBuf<int> flag;
+    DevBuf<unsigned long long> cnt;
+};
+
 struct letkf_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -332,15 +345,10 @@ struct letkf_ctx {
     // (k x k FP32), g or wbar (FP64), lambda
     DevBuf<float> d_mA, d_mX, d_mlam;
     DevBuf<double> d_mg;
-    // the FP64 form's tensor-core path (letkf_f64.cu; it shares d_mA, d_mX,
-    // d_mlam and d_mg): A or T' as integers, the largest diagonal element of
-    // A', flags and list of the problems left to k_core_fp64 and the exponents
-    // of A, counters, row maxima of y; k = 96, 128:
-    // scratch of each CTA
-    DevBuf<long long> d_fA, d_fscr;
-    DevBuf<float> d_famax, d_frowmax;
-    DevBuf<int> d_fflag;
-    DevBuf<unsigned long long> d_fcnt;
+    // the FP64 form's runs, and the batched core: its problems are the
+    // caller's, and a set of its own leaves the buffers of a captured run where
+    // the graph has them
+    LgF64Scratch f64, f64_batch;
     DevBuf<float> d_ys32;         // yb * sqrt(rinv) in FP32 (mixed precision)
     DevBuf<float> d_rinvf;
     DevBuf<float> d_oef;          // mixed form: sqrt(rdiaginv) dep per obs
@@ -387,6 +395,7 @@ struct letkf_ctx {
     DevBuf<double> d_bhx, d_bdep, d_brloc;
     DevBuf<float> d_brdi;
     DevBuf<int64_t> d_boff;
+    DevBuf<int32_t> d_bcnt;
     // status
     DevBuf<unsigned int> d_status;
     DevBuf<unsigned long long> d_counters;
