@@ -643,6 +643,8 @@ void fill_stats(letkf_ctx *ctx, const unsigned long long *cnt)
     s.sched_chunk = ctx->sched_chunk;
     s.n_windows = ctx->last_windows;
     s.precision = ctx->params.precision;
+    ctx->general_problems = (int64_t)cnt[LG_CNT_GENERAL];
+    ctx->general_columns = (int64_t)cnt[LG_CNT_GENCOLS];
 }
 
 }  // namespace
@@ -1332,6 +1334,10 @@ int letkf_gpu_core_batch(letkf_ctx *ctx, int64_t nb, const int64_t *offsets, con
     dw.release();
     // the status and the counters of the last run were overwritten
     ctx->have_run = false;
+    if (e == cudaSuccess && !rc) {
+        ctx->general_problems = (int64_t)cnt2[LG_CNT_GENERAL];
+        ctx->general_columns = 0;
+    }
     if (e != cudaSuccess) return set_err(ctx, LETKF_ERR_CUDA, cudaGetErrorString(e));
     if (rc) return rc;
     if (st & LG_ST_TIMEOUT)
@@ -1345,6 +1351,14 @@ int letkf_gpu_get_stats(letkf_ctx *ctx, letkf_stats *stats)
 {
     if (!ctx || !stats) return LETKF_ERR_INVALID;
     *stats = ctx->stats;
+    return LETKF_OK;
+}
+
+int letkf_gpu_general_counts(letkf_ctx *ctx, int64_t *problems, int64_t *columns)
+{
+    if (!ctx || !problems || !columns) return LETKF_ERR_INVALID;
+    *problems = ctx->general_problems;
+    *columns = ctx->general_columns;
     return LETKF_OK;
 }
 

@@ -111,6 +111,8 @@ k_core_fp64(LgGrid g, LgParams prm, LgRowSrc src, const int64_t *__restrict__ lo
         atomicAdd(&counters[LG_CNT_SUMSWEEP], ls.fold[LG_CNT_SUMSWEEP]);
     }
     const int64_t nitem = ls.list ? (int64_t)*ls.n : ncubes - prm.cube0;
+    if (K >= 32 && blockIdx.x == 0 && tid == 0)
+        atomicAdd(&counters[LG_CNT_GENERAL], (unsigned long long)(nitem * (ls.list ? 1 : nvb)));
     for (int64_t item = blockIdx.x; item < nitem; item += gridDim.x) {
         const int64_t prob = ls.list ? ls.q0 + ls.list[item] : 0;
         const int64_t cube = ls.list ? prob / ls.nvb : prm.cube0 + item;
@@ -409,7 +411,8 @@ template <int K>
 __global__ void __launch_bounds__(kT)
 k_overlap_update(LgGrid g, LgParams prm, const double *__restrict__ trans, const double *__restrict__ xb,
                  const double *__restrict__ axb, double *__restrict__ xa, double *__restrict__ axa,
-                 const int *__restrict__ list, const unsigned long long *__restrict__ nlist)
+                 const int *__restrict__ list, const unsigned long long *__restrict__ nlist,
+                 unsigned long long *__restrict__ counters)
 {
     extern __shared__ double Ts[];               // Ts[l * (K + 1) + e] = trans(l, e)
     constexpr int LDT = K + 1, PER = (K + 31) / 32;
@@ -417,6 +420,7 @@ k_overlap_update(LgGrid g, LgParams prm, const double *__restrict__ trans, const
     const int n = g.n, step = prm.cube_step, cn = prm.cube_n;
     // every column, or the listed ones
     const int64_t ncol = list ? (int64_t)*nlist : (int64_t)g.nlat * g.nlon;
+    if (K >= 32 && blockIdx.x == 0 && tid == 0) atomicAdd(&counters[LG_CNT_GENCOLS], (unsigned long long)ncol);
     for (int64_t ci = blockIdx.x; ci < ncol; ci += gridDim.x) {
         const int64_t c = list ? list[ci] : ci;
         const int jj = (int)(c % g.nlat), ii = (int)(c / g.nlat);
@@ -486,7 +490,7 @@ cudaError_t launch_overlap(letkf_ctx *ctx, const LgGrid &g, const double *xb, co
     const unsigned blocks = list ? 512u : (unsigned)(ncol < (1 << 30) ? ncol : (1 << 30));
     lg_count_launch();
     k_overlap_update<K><<<blocks, kT, smem, ctx->stream>>>(g, lg_params(ctx), ctx->d_trans.p, xb, axb, xa, axa, list,
-                                                           nlist);
+                                                           nlist, ctx->d_counters.p);
     return cudaGetLastError();
 }
 

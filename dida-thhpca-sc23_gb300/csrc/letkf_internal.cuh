@@ -62,6 +62,8 @@ enum {
     LG_CNT_SUMSWEEP,
     LG_CNT_ILLCOND,
     LG_CNT_QUEUE,         // work-queue cursor of the mixed core
+    LG_CNT_GENERAL,       // FP64 form, k >= 32: problems that k_core_fp64 solved
+    LG_CNT_GENCOLS,       // and overlapped columns that k_overlap_update averaged
     LG_CNT_N
 };
 
@@ -411,6 +413,7 @@ struct letkf_ctx {
     cudaEvent_t stg_ev[kStages][2][kStageMarks] = {};
     int stg_n[kStages] = {};
     letkf_stats stats{};
+    int64_t general_problems = 0, general_columns = 0;      // LG_CNT_GENERAL, LG_CNT_GENCOLS of the last call
     std::string last_error;
 
     // Host copies beside the analysis (letkf_gpu_run with host pointers): the

@@ -43,7 +43,7 @@ EXPORTED = [
     "letkf_gpu_run_halo", "letkf_gpu_set_schedule", "letkf_gpu_set_host_read",
     "letkf_gpu_synchronize", "letkf_gpu_obs_operator", "letkf_gpu_local_obs",
     "letkf_gpu_last_trans", "letkf_gpu_core_batch", "letkf_gpu_get_stats",
-    "letkf_gpu_last_error", "letkf_gpu_destroy", "letkf_gpu_launch_count",
+    "letkf_gpu_general_counts", "letkf_gpu_last_error", "letkf_gpu_destroy", "letkf_gpu_launch_count",
     "letkf_gpu_core_batch_noalloc", "letkf_decomp_dims", "letkf_gpu_autotune",
     "letkf_batch_create", "letkf_batch_launch", "letkf_batch_sync", "letkf_batch_launches",
     "letkf_batch_destroy", "letkf_gpu_set_list_limit", "letkf_gpu_set_cube_range", "letkf_gpu_run_members",
@@ -135,6 +135,7 @@ def load_library(path: str = LIB_PATH):
     L.letkf_gpu_last_trans.argtypes = [vp, vp, i64, vp, vp]
     L.letkf_gpu_core_batch.argtypes = [vp, i64, vp, vp, vp, vp, vp, vp, vp]
     L.letkf_gpu_get_stats.argtypes = [vp, C.POINTER(Stats)]
+    L.letkf_gpu_general_counts.argtypes = [vp, C.POINTER(i64), C.POINTER(i64)]
     L.letkf_gpu_last_error.argtypes = [vp]
     L.letkf_gpu_last_error.restype = C.c_char_p
     L.letkf_gpu_destroy.argtypes = [vp]
@@ -517,6 +518,13 @@ class LetkfGPU:
         s = Stats()
         self._check(self.L.letkf_gpu_get_stats(self.h, C.byref(s)), "get_stats")
         return s.as_dict()
+
+    def general_counts(self):
+        """(problems, columns) of the last call that the FP64 form's general kernels
+        took instead of the tensor-core path."""
+        p, c = C.c_int64(), C.c_int64()
+        self._check(self.L.letkf_gpu_general_counts(self.h, C.byref(p), C.byref(c)), "general_counts")
+        return p.value, c.value
 
 
 def struct_atm2endnn(xb, xb2, ens_start=1, n_start=1, stream=None):

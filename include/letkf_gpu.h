@@ -415,6 +415,15 @@ int64_t letkf_batch_launches(letkf_batch *batch);   /* kernels per replay */
 int letkf_batch_destroy(letkf_batch *batch);
 
 int letkf_gpu_get_stats(letkf_ctx *ctx, letkf_stats *stats);
+
+/* FP64 form, ensembles of 32 and more: the local problems (cubes, or level
+ * blocks of cubes) of the last run, batched core or batch sync that the general
+ * FP64 kernel solved instead of the tensor-core path (operands that are not
+ * finite or out of its range, a badly conditioned A', device arrays between
+ * 16-byte boundaries, no memory for its buffers), about 20 times as slow, and the
+ * columns of overlapped cubes averaged one cube at a time likewise.  No
+ * counterpart in the reference.                                              */
+int letkf_gpu_general_counts(letkf_ctx *ctx, int64_t *problems, int64_t *columns);
 const char *letkf_gpu_last_error(letkf_ctx *ctx);
 int letkf_gpu_destroy(letkf_ctx *ctx);
 
