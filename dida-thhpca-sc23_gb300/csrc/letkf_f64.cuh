@@ -84,9 +84,9 @@ struct ListSrc {
 };
 
 // The fixed point of a list: Yhat 2^sY and e 2^sE rounded to integers, sums of
-// products in units of 2^sh of level 5.
+// products in units of 2^sh of level 5 (A) and 2^shG (g).
 struct ListScale {
-    int sY, sE, sh;
+    int sY, sE, sh, shG;
     bool bad;                  // not finite, or out of range
 };
 
@@ -137,7 +137,6 @@ __device__ __forceinline__ ListScale list_scale(const ListSrc &L, int first, dou
         se += __uint_as_float(wm[3][i]);
     }
     ListScale r;
-    r.bad = my >= 0x7e000000u || me >= 0x7e000000u || L.p > (1 << 21);
     // the sum of squares in units of the largest: with at most 16 in any 128
     // observations the first digit may have one bit more
     const float mf = __uint_as_float(my), mef = __uint_as_float(me), n = (float)L.p;
@@ -145,11 +144,19 @@ __device__ __forceinline__ ListScale list_scale(const ListSrc &L, int first, dou
     if (!(ratio < n) || mf < 1e-15f) ratio = n;
     const float part = L.p > 128 ? 256.0f / n : 1.0f;
     const int more = ratio * part <= 15.9f ? 1 : 0;
-    const int more_e = mef > 1e-15f && 1.001f * (se / mef) / mef * part <= 15.9f ? 1 : 0;
+    float ratio_e = 1.001f * (se / mef) / mef;
+    if (!(ratio_e < n) || mef < 1e-15f) ratio_e = n;
+    const int more_e = ratio_e * part <= 15.9f ? 1 : 0;
     r.sY = 48 + more - lg_exp2f_bits(__float_as_uint(mf * 1.01f));
     r.sE = 48 + more_e - lg_exp2f_bits(__float_as_uint(mef * 1.01f));
     // A <= ratio 2^(98 + 2 more): 2 A 2^-(30 + sh) < 2^61
     r.sh = 8 + 2 * more + max(1, lg_exp2f_bits(__float_as_uint(fmaxf(ratio, 1.0f))) + 1);
+    // |g| <= sqrt(ratio ratio_e) 2^(98 + more + more_e) (Cauchy-Schwarz): a few
+    // strong rows among many weak ones have a small ratio of Yhat beside a large
+    // one of e, and g needs more room than A's unit leaves
+    const float rg = sqrtf(fmaxf(ratio, 1.0f)) * sqrtf(fmaxf(ratio_e, 1.0f)) * 1.001f;
+    r.shG = 8 + more + more_e + max(1, lg_exp2f_bits(__float_as_uint(rg)) + 1);
+    r.bad = my >= 0x7e000000u || me >= 0x7e000000u || r.sh > 30 || r.shG > 30;
     return r;
 }
 
