@@ -8,7 +8,6 @@
 namespace {
 
 constexpr int kTF = 512;                  // threads of the kernels below
-constexpr int kFlush = 2;                 // chunks of 64 observations per exact accumulation
 constexpr int kMaxIter = 8;               // most corrections of T
 
 // Storage size of a problem's k x k matrices between the launches.
@@ -87,13 +86,15 @@ struct ListSrc {
 // products in units of 2^sh of level 5 (A) and 2^shG (g).
 struct ListScale {
     int sY, sE, sh, shG;
+    bool pairs;                // the first digits' squares over any 128 observations stay below 2^24
     bool bad;                  // not finite, or out of range
 };
 
-// Scales from bounds over the whole list: the largest |Yhat| and |e| and the
-// sums of squares of e and of the rows' largest |Yhat|; thread t < first brings
-// entry t, the others are read here without the vertical weight (at most 1).
-// wm: 4 x 16 words of shared memory.  Called by all kTF threads.
+// Scales from bounds over the whole list: the largest |Yhat| and |e|, and the
+// sums of squares of e and of the rows' largest |Yhat| over the list and over
+// every group of 128 observations (what two chunks sum); thread t < first brings
+// entry t, the others are read here (a vertical weight from FP32, rounded up).
+// wm: 6 x 16 words of shared memory.  Called by all kTF threads.
 __device__ __forceinline__ ListScale list_scale(const ListSrc &L, int first, double e_s, double e_sd, float e_rm,
                                                 unsigned (*wm)[kTF / 32])
 {
@@ -101,52 +102,81 @@ __device__ __forceinline__ ListScale list_scale(const ListSrc &L, int first, dou
     const LgRowSrc &src = L.src;
     const float y0 = e_rm * (__double2float_ru(e_s) * 1.0001f), d0 = __double2float_ru(fabs(e_sd));
     unsigned my = __float_as_uint(y0) & 0x7fffffffu, me = __float_as_uint(d0) & 0x7fffffffu;
-    float sq = y0 * y0, se = d0 * d0;
-    for (int i = tid + first; i < L.p; i += kTF) {
-        const int64_t li = L.off + i;
-        const int64_t gi = src.batch ? li : (int64_t)src.lidx[li];
-        const float rd = src.batch ? src.brdi[li] : src.rinvf[gi];
-        const double rl = src.batch ? src.brloc[li] : src.lrloc[li];
-        const float s = sqrtf(rd * (float)rl) * 1.0001f;
-        const float d = fabsf((float)(src.batch ? src.bdep[li] : src.dep[gi])) * s, y = L.rowmax[gi] * s;
+    auto warp_sum = [](float x) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        return x;
+    };
+    // a warp's 32 entries are a quarter of a group; `first` and kTF are whole
+    // groups, so warps 4 g .. 4 g + 3 always share one: the largest sums of
+    // each warp bound every group's
+    float sq = warp_sum(y0 * y0), se = warp_sum(d0 * d0), gq = sq, ge = se;
+    for (int i0 = first + 32 * warp; i0 < L.p; i0 += kTF) {
+        float y = 0.0f, d = 0.0f;
+        if (i0 + lane < L.p) {
+            const int64_t li = L.off + i0 + lane;
+            const int64_t gi = src.batch ? li : (int64_t)src.lidx[li];
+            const float rd = src.batch ? src.brdi[li] : src.rinvf[gi];
+            float rl = (float)(src.batch ? src.brloc[li] : src.lrloc[li]);
+            if (L.vertical) {
+                const float z = (float)(fabs(L.lnp - src.olnp[gi]) / L.vert_dist);
+                // (FP32 next to the cut-off is good to 1e-6 of the weight at zero)
+                rl *= L.gcv ? lg_schr2f(z) + 4e-6f : z > 2.0001f ? 0.0f : 1.0f;
+            }
+            const float s = sqrtf(rd) * sqrtf(rl) * 1.0001f;
+            d = fabsf((float)(src.batch ? src.bdep[li] : src.dep[gi])) * s;
+            y = L.rowmax[gi] * s;
+        }
         my = max(my, __float_as_uint(y) & 0x7fffffffu);
         me = max(me, __float_as_uint(d) & 0x7fffffffu);
-        sq = fmaf(y, y, sq);
-        se = fmaf(d, d, se);
+        const float wq = warp_sum(y * y), we = warp_sum(d * d);
+        sq += wq;
+        se += we;
+        gq = fmaxf(gq, wq);
+        ge = fmaxf(ge, we);
     }
     my = __reduce_max_sync(0xffffffffu, my);
     me = __reduce_max_sync(0xffffffffu, me);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        sq += __shfl_xor_sync(0xffffffffu, sq, o);
-        se += __shfl_xor_sync(0xffffffffu, se, o);
-    }
     if (lane == 0) {
         wm[0][warp] = my;
         wm[1][warp] = me;
         wm[2][warp] = __float_as_uint(sq);
         wm[3][warp] = __float_as_uint(se);
+        wm[4][warp] = __float_as_uint(gq);
+        wm[5][warp] = __float_as_uint(ge);
     }
     __syncthreads();
-    sq = se = 0.0f;
+    sq = se = gq = ge = 0.0f;
 #pragma unroll
-    for (int i = 0; i < kTF / 32; i++) {
-        my = max(my, wm[0][i]);
-        me = max(me, wm[1][i]);
-        sq += __uint_as_float(wm[2][i]);
-        se += __uint_as_float(wm[3][i]);
+    for (int g = 0; g < kTF / 128; g++) {
+        float a = 0.0f, b = 0.0f;
+#pragma unroll
+        for (int i = 4 * g; i < 4 * g + 4; i++) {
+            my = max(my, wm[0][i]);
+            me = max(me, wm[1][i]);
+            sq += __uint_as_float(wm[2][i]);
+            se += __uint_as_float(wm[3][i]);
+            a += __uint_as_float(wm[4][i]);
+            b += __uint_as_float(wm[5][i]);
+        }
+        gq = fmaxf(gq, a);
+        ge = fmaxf(ge, b);
     }
     ListScale r;
-    // the sum of squares in units of the largest: with at most 16 in any 128
-    // observations the first digit may have one bit more
+    // the sums of squares in units of the largest (the worst case where FP32
+    // cannot hold them)
     const float mf = __uint_as_float(my), mef = __uint_as_float(me), n = (float)L.p;
-    float ratio = 1.001f * (sq / mf) / mf;
-    if (!(ratio < n) || mf < 1e-15f) ratio = n;
-    const float part = L.p > 128 ? 256.0f / n : 1.0f;
-    const int more = ratio * part <= 15.9f ? 1 : 0;
-    float ratio_e = 1.001f * (se / mef) / mef;
-    if (!(ratio_e < n) || mef < 1e-15f) ratio_e = n;
-    const int more_e = ratio_e * part <= 15.9f ? 1 : 0;
+    auto units = [](float sum, float most, float worst) {
+        const float u = 1.001f * (sum / most) / most;
+        return u < worst && most >= 1e-15f ? u : worst;
+    };
+    const float ratio = units(sq, mf, n), ratio_e = units(se, mef, n);
+    const float group = units(gq, mf, 128.0f), group_e = units(ge, mef, 128.0f);
+    // first digits of at most 512; with at most 16 units in any 128 observations
+    // they may have one bit more (their squares then stay below 2^24), with more
+    // than 64 they are summed 64 observations at a time
+    const int more = group <= 15.9f ? 1 : 0, more_e = group_e <= 15.9f ? 1 : 0;
+    r.pairs = group <= 63.0f && group_e <= 63.0f;
     r.sY = 48 + more - lg_exp2f_bits(__float_as_uint(mf * 1.01f));
     r.sE = 48 + more_e - lg_exp2f_bits(__float_as_uint(mef * 1.01f));
     // A <= ratio 2^(98 + 2 more): 2 A 2^-(30 + sh) < 2^61
