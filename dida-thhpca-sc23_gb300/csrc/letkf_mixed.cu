@@ -110,12 +110,15 @@ struct MCfg {
                                           ? 2 * (size_t)TILE
                                           : 2 * (size_t)K * (K + 1) * sizeof(float)) + 1023) & ~(size_t)1023;
     static constexpr size_t SMEM1 = 1024 + AREA1 + B1 + VEC;
-    // the update launch without the members (ST 3): the xb and T tiles (48 KB),
-    // the epilogue's exchange rows, and the mean-increment partials in place of
-    // B1 (T is read from its slot in global memory): three CTAs per SM
+    // the update launch (ST 3): the xb and T tiles (48 KB), the epilogue's
+    // exchange rows, and the mean-increment partials (members: and the squared
+    // perturbations') in place of B1 (T is read from its slot in global memory):
+    // three CTAs per SM
     static constexpr size_t AREA3 = 53 * 1024;
     static constexpr size_t B13 = sizeof(double) * 128 * (K / 8);
+    static constexpr size_t SQ3 = sizeof(float) * 128 * (K / 8);
     static constexpr size_t SMEM3 = 1024 + AREA3 + B13 + VEC;
+    static constexpr size_t SMEM3M = SMEM3 + SQ3;
     static_assert(49152 + 128 * 9 * sizeof(float) <= AREA3, "update tiles and exchange rows");
     static_assert(2 * (size_t)K * (K + 1) * sizeof(float) <= AREA1, "Dhh and Dlh must fit over the tiles");
     static_assert(AREA1 % 1024 == 0, "1024-byte aligned tiles");
@@ -143,32 +146,45 @@ struct MCfg {
 // xa (xb from the row's BF16 hi/lo tile, 2^-17 of xb), else the background
 // members themselves; spread_b = sqrt(sum xb^2 / ens) from the staging's
 // partial sums, spread_a = sqrt(sum (member - axa)^2 / ens).
+struct MembersRow {
+    bool blend;
+    double cst;                // gamma1 mb + gamma2 ma
+    float df, g1, g2, sb;      // cst - ma; sum of squared background perturbations
+};
+
 template <int K>
-__device__ __forceinline__ void members_epilogue(const LgParams &prm, const LgGrid &g, int64_t col, int r,
-                                                 const double *xin_row, const unsigned char *t_hi,
-                                                 const unsigned char *t_lo, double mb, double incr, float meanf,
-                                                 const float *v, const float *sqp, double *dst, int64_t row)
+__device__ __forceinline__ MembersRow members_row(const LgParams &prm, const LgGrid &g, int64_t col, int r, double mb,
+                                                  double incr, const float *sqp)
 {
-    const float fk = (float)K;
-    float sb = 0.0f;
+    MembersRow m;
+    m.sb = 0.0f;
 #pragma unroll
-    for (int c = 0; c < K / 8; c++) sb += sqp[c * 128 + r];
+    for (int c = 0; c < K / 8; c++) m.sb += sqp[c * 128 + r];
     const double ma = mb + incr;
-    const bool blend = fabs((double)g.glat[col % g.nlat]) <= prm.polar;
-    if (!blend) {
-        for (int e = 0; e < K; e += 2)
-            *reinterpret_cast<double2 *>(dst + e) = *reinterpret_cast<const double2 *>(xin_row + e);
-        prm.spb[row] = sqrt((double)(sb / fk));
-        prm.spa[row] = sqrt((double)(sb / fk));
+    m.blend = fabs((double)g.glat[col % g.nlat]) <= prm.polar;
+    m.cst = prm.gamma1 * mb + prm.gamma2 * ma;
+    m.df = (float)(m.cst - ma);
+    m.g1 = (float)prm.gamma1;
+    m.g2 = (float)prm.gamma2;
+    return m;
+}
+
+// Members 8 c0 .. 8 c0 + N - 1 of the row (v, xin and dst start there): written to
+// dst, and v becomes their perturbation parts.
+template <int N>
+__device__ __forceinline__ void members_half(const MembersRow &m, int r, int c0, const double *xin,
+                                             const unsigned char *t_hi, const unsigned char *t_lo, float meanf,
+                                             float *v, double *dst)
+{
+    if (!m.blend) {
+        for (int e = 0; e < N; e += 2)
+            *reinterpret_cast<double2 *>(dst + e) = *reinterpret_cast<const double2 *>(xin + e);
         return;
     }
-    const double cst = prm.gamma1 * mb + prm.gamma2 * ma;
-    const float df = (float)(cst - ma), g1 = (float)prm.gamma1, g2 = (float)prm.gamma2;
-    float sa = 0.0f;
 #pragma unroll
-    for (int c = 0; c < K / 8; c++) {
-        const uint4 h = *reinterpret_cast<const uint4 *>(t_hi + lg_sw128_offset(r, c));
-        const uint4 l = *reinterpret_cast<const uint4 *>(t_lo + lg_sw128_offset(r, c));
+    for (int c = 0; c < N / 8; c++) {
+        const uint4 h = *reinterpret_cast<const uint4 *>(t_hi + lg_sw128_offset(r, c0 + c));
+        const uint4 l = *reinterpret_cast<const uint4 *>(t_lo + lg_sw128_offset(r, c0 + c));
         const uint32_t hw[4] = {h.x, h.y, h.z, h.w}, lw[4] = {l.x, l.y, l.z, l.w};
 #pragma unroll
         for (int q = 0; q < 4; q++) {
@@ -176,13 +192,20 @@ __device__ __forceinline__ void members_epilogue(const LgParams &prm, const LgGr
             const float b0 = __uint_as_float(hw[q] << 16) + __uint_as_float(lw[q] << 16);
             const float b1 = __uint_as_float(hw[q] & 0xffff0000u) + __uint_as_float(lw[q] & 0xffff0000u);
             const int e = 8 * c + 2 * q;
-            const float d0 = fmaf(g1, b0, g2 * (v[e] - meanf)), d1 = fmaf(g1, b1, g2 * (v[e + 1] - meanf));
-            sa = fmaf(df + d0, df + d0, fmaf(df + d1, df + d1, sa));
-            *reinterpret_cast<double2 *>(dst + e) = make_double2(cst + lg_f2d_bits(d0), cst + lg_f2d_bits(d1));
+            v[e] = fmaf(m.g1, b0, m.g2 * (v[e] - meanf));
+            v[e + 1] = fmaf(m.g1, b1, m.g2 * (v[e + 1] - meanf));
+            *reinterpret_cast<double2 *>(dst + e) = make_double2(m.cst + lg_f2d_bits(v[e]), m.cst + lg_f2d_bits(v[e + 1]));
         }
     }
-    prm.spb[row] = sqrt((double)(sb / fk));
-    prm.spa[row] = sqrt((double)(sa / fk));
+}
+
+// sa plus the squares of (member - axa) of members_half's members, in order.
+template <int N>
+__device__ __forceinline__ float members_sum(const MembersRow &m, const float *v, float sa)
+{
+#pragma unroll
+    for (int e = 0; e < N; e += 2) sa = fmaf(m.df + v[e], m.df + v[e], fmaf(m.df + v[e + 1], m.df + v[e + 1], sa));
+    return sa;
 }
 
 // ST selects the stages a launch runs: 0 all of them; 1 the A build only
@@ -193,7 +216,7 @@ __device__ __forceinline__ void members_epilogue(const LgParams &prm, const LgGr
 // MEM: the fused members run (LgParams::members; stages 0 and 3), a separate
 // instantiation so the plain update keeps its registers.
 template <int K, int ST, bool MEM = false>
-__global__ void __launch_bounds__(kT, (ST == 1 || (ST == 3 && !MEM)) ? 3 : 2)
+__global__ void __launch_bounds__(kT, (ST == 1 || ST == 3) ? 3 : 2)
 k_core_mixed(LgGrid g, LgParams prm, const float *__restrict__ ys32, const int32_t *__restrict__ lidx,
              const float2 *__restrict__ lmeta, const int *__restrict__ queue, int nchunks, int chunk,
              const int64_t *__restrict__ loff, const int32_t *__restrict__ lcnt, int64_t ncubes,
@@ -207,9 +230,9 @@ k_core_mixed(LgGrid g, LgParams prm, const float *__restrict__ ys32, const int32
     constexpr int CH = C::CH;
     extern __shared__ unsigned char smem_raw[];
     unsigned char *area = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    constexpr bool U3 = ST == 3 && !MEM;      // the compact update layout (MCfg::SMEM3)
+    constexpr bool U3 = ST == 3;              // the compact update layout (MCfg::SMEM3)
     double *B1 = reinterpret_cast<double *>(area + (ST == 1 ? C::AREA1 : U3 ? C::AREA3 : C::AREA));
-    double *gv = B1 + (U3 ? 128 * (K / 8) : K * K);
+    double *gv = B1 + (U3 ? 128 * (K / 8) + (MEM ? (int)(C::SQ3 / sizeof(double)) : 0) : K * K);
     double *wbar = gv + K;
     double *misc = wbar + K;       // 2K
     double *inc = misc + 2 * K;    // 128
@@ -870,9 +893,9 @@ k_core_mixed(LgGrid g, LgParams prm, const float *__restrict__ ys32, const int32
         // after T in the space of A' (free in this phase)
         double *incp = U3 ? B1 : reinterpret_cast<double *>(T32 + K * K);
         // fused members run: squared perturbations summed over 8 members,
-        // [c][row], beside the mean-increment partials (k >= 48) or after the
-        // warm-start vectors (k = 32)
-        constexpr bool SQ_IN_B1 = 128 * K + 64 * K <= 4 * K * K;
+        // [c][row], beside the mean-increment partials (k >= 48, and the update
+        // launch) or after the warm-start vectors (k = 32)
+        constexpr bool SQ_IN_B1 = U3 || 128 * K + 64 * K <= 4 * K * K;
         float *sqp = SQ_IN_B1 ? reinterpret_cast<float *>(incp + 128 * (K / 8))
                               : reinterpret_cast<float *>(area + 49152 + K * K * sizeof(float));
         static_assert(128 * K <= 4 * K * K, "mean-increment partials must fit beside T");
@@ -974,7 +997,7 @@ k_core_mixed(LgGrid g, LgParams prm, const float *__restrict__ ys32, const int32
                         break;
                     }
                     lg_tc_fence_after();
-                    if constexpr (ST == 3 && !MEM) {
+                    if constexpr (ST == 3) {
                         // all 8 warps: warp w reads row quadrant w % 4 (the
                         // tensor-memory lanes it may access) and members
                         // (w / 4) K/2 .. +K/2 - 1.  The member mean keeps the
@@ -1009,7 +1032,28 @@ k_core_mixed(LgGrid g, LgParams prm, const float *__restrict__ ys32, const int32
                                              (float)K;
                         }
                         __syncthreads();
-                        if (r < R) {
+                        if constexpr (MEM) {
+                            // the spread's sum of squares continues the first half's
+                            const bool on = r < R;
+                            MembersRow mr{};
+                            if (on) {
+                                double incr = incp[r];
+#pragma unroll
+                                for (int c = 1; c < K / 8; c++) incr += incp[c * 128 + r];
+                                mr = members_row<K>(prm, g, col, r, inc[r], incr, sqp);
+                                const int64_t at = (int64_t)(r0 + r) * K + hh * (K / 2);
+                                members_half<K / 2>(mr, r, hh * (K / 16), xbc + at, xa_hi, xa_lo, xch[r * 9 + 8], v,
+                                                    xac + at);
+                                if (hh == 0) xch[r * 9] = members_sum<K / 2>(mr, v, 0.0f);
+                            }
+                            __syncthreads();
+                            if (on && hh == 1) {
+                                const int64_t row = col * n + r0 + r;
+                                const float sa = members_sum<K / 2>(mr, v, xch[r * 9]);
+                                prm.spb[row] = sqrt((double)(mr.sb / (float)K));
+                                prm.spa[row] = sqrt((double)((mr.blend ? sa : mr.sb) / (float)K));
+                            }
+                        } else if (r < R) {
                             const float meanf = xch[r * 9 + 8];
                             const int64_t row = col * n + r0 + r;
                             double *dst = xac + (int64_t)(r0 + r) * K + hh * (K / 2);
@@ -1054,8 +1098,11 @@ k_core_mixed(LgGrid g, LgParams prm, const float *__restrict__ ys32, const int32
                                     *reinterpret_cast<double2 *>(dst + e) =
                                         make_double2(lg_f2d_bits(v[e] - meanf), lg_f2d_bits(v[e + 1] - meanf));
                             } else {
-                                members_epilogue<K>(prm, g, col, r, xbc + (int64_t)(r0 + r) * K, xa_hi, xa_lo,
-                                                    inc[r], incr, meanf, v, sqp, dst, row);
+                                const MembersRow mr = members_row<K>(prm, g, col, r, inc[r], incr, sqp);
+                                members_half<K>(mr, r, 0, xbc + (int64_t)(r0 + r) * K, xa_hi, xa_lo, meanf, v, dst);
+                                const float sa = members_sum<K>(mr, v, 0.0f);
+                                prm.spb[row] = sqrt((double)(mr.sb / (float)K));
+                                prm.spa[row] = sqrt((double)((mr.blend ? sa : mr.sb) / (float)K));
                             }
                         }
                     }
@@ -1787,9 +1834,9 @@ template <int K, int ST>
 cudaError_t launch_stage(letkf_ctx *ctx, const LgGrid &g, const double *xb, const double *axb, double *xa,
                          double *axa, double *trans_out, double *w_out, int chunk, int nchunks, int nsm)
 {
-    // the update without the members takes the compact layout
-    const bool u3 = ST == 3 && !ctx->members_on;
-    const size_t smem = ST == 1 ? MCfg<K>::SMEM1 : u3 ? MCfg<K>::SMEM3 : MCfg<K>::SMEM;
+    const size_t smem = ST == 1   ? MCfg<K>::SMEM1
+                        : ST == 3 ? (ctx->members_on ? MCfg<K>::SMEM3M : MCfg<K>::SMEM3)
+                                  : MCfg<K>::SMEM;
     auto kern = (ST != 1 && ctx->members_on) ? k_core_mixed<K, ST, ST != 1> : k_core_mixed<K, ST, false>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -1799,9 +1846,9 @@ cudaError_t launch_stage(letkf_ctx *ctx, const LgGrid &g, const double *xb, cons
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
     // CTAs per SM: as many as the launch bounds give registers for (2; 3 for
-    // the A build and the plain update) when their shared memory (plus the 1 KB the system keeps per
-    // CTA and the static barriers) fits
-    int per_sm = (ST == 1 || u3) ? 3 : 2;
+    // the A build and the update) when their shared memory (plus the 1 KB the
+    // system keeps per CTA and the static barriers) fits
+    int per_sm = (ST == 1 || ST == 3) ? 3 : 2;
     while (per_sm > 1 && (size_t)per_sm * (smem + 1024 + 64) > (size_t)smem_sm) per_sm--;
     // persistent grid: each CTA allocates its tensor memory once
     const int64_t want = (int64_t)nsm * per_sm;
