@@ -884,6 +884,14 @@ int letkf_gpu_set_list_limit(letkf_ctx *ctx, int64_t max_entries)
     return LETKF_OK;
 }
 
+int letkf_gpu_set_scratch_limit(letkf_ctx *ctx, int64_t bytes)
+{
+    if (!ctx) return LETKF_ERR_INVALID;
+    if (bytes < 0) return set_err(ctx, LETKF_ERR_INVALID, "negative scratch limit");
+    ctx->scratch_limit = bytes;
+    return LETKF_OK;
+}
+
 int letkf_gpu_set_cube_range(letkf_ctx *ctx, int64_t first, int64_t count)
 {
     if (!ctx) return LETKF_ERR_INVALID;

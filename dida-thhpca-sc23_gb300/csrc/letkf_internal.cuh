@@ -351,6 +351,7 @@ struct letkf_ctx {
     // caller's, and a set of its own leaves the buffers of a captured run where
     // the graph has them
     LgF64Scratch f64, f64_batch;
+    int64_t scratch_limit = 0;    // most bytes of either (0: what fits; letkf_gpu_set_scratch_limit)
     DevBuf<float> d_ys32;         // yb * sqrt(rinv) in FP32 (mixed precision)
     DevBuf<float> d_rinvf;
     DevBuf<float> d_oef;          // mixed form: sqrt(rdiaginv) dep per obs

@@ -207,9 +207,10 @@ extern "C" int letkf_gpu_run_members(letkf_ctx *ctx, const double *xb_in, const 
     // The FP64 form's tensor-core path (letkf_f64.cu) takes the split state:
     // its analysis with two passes over the state is far shorter than the
     // fused k_core_fp64 (4 degrees, k = 64, 4,050 columns: 4.9 against 81 ms
-    // on the device).  Where the split state does not fit the device the
-    // fused form stays.
-    if (fused && !lg_is_mixed(ctx->params.precision) && lg_f64_supports(k)) {
+    // on the device).  Where the split state does not fit the device, or the
+    // context's limit, the fused form stays.
+    if (fused && !lg_is_mixed(ctx->params.precision) && lg_f64_supports(k) &&
+        (ctx->scratch_limit == 0 || 16 * (nstate + nmean) <= (size_t)ctx->scratch_limit)) {
         cudaError_t e = ctx->d_xb.reserve(nstate);
         if (e == cudaSuccess) e = ctx->d_axb.reserve(nmean);
         if (e == cudaSuccess) e = ctx->d_xa.reserve(nstate);

@@ -860,6 +860,15 @@ cudaError_t launch_wide(letkf_ctx *ctx, const LgGrid &g, const double *xb, const
     // chunks and the results do not depend on the blocking
     int64_t step = std::max(kWideCubes, unit);
     auto block_end = [&](int64_t b) { return std::min(w1, (b / step + 1) * step); };
+    // larger blocks than what is held only where the device has room for them: one
+    // that is short of memory keeps its buffers from run to run
+    const size_t kk = (size_t)K * K, cube_bytes = 2 * kk * sizeof(float) + K * sizeof(double);
+    const int64_t held = (int64_t)std::min(std::min(ctx->d_mA.n, ctx->d_mX.n) / kk, ctx->d_mg.n / K);
+    size_t fr = 0, tot = 0;
+    if (std::min(step, w1 - w0) > held && cudaMemGetInfo(&fr, &tot) == cudaSuccess)
+        while (step > unit && std::min(step, w1 - w0) > held &&
+               (size_t)std::min(step, w1 - w0) * cube_bytes > fr + (size_t)held * cube_bytes)
+            step /= 2;
     for (;; step /= 2) {
         const size_t most = (size_t)std::min(step, w1 - w0);
         e = ctx->d_mA.reserve(most * K * K);

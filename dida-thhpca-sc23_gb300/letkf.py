@@ -43,7 +43,7 @@ EXPORTED = [
     "letkf_gpu_run_halo", "letkf_gpu_set_schedule", "letkf_gpu_set_host_read",
     "letkf_gpu_synchronize", "letkf_gpu_obs_operator", "letkf_gpu_local_obs",
     "letkf_gpu_last_trans", "letkf_gpu_core_batch", "letkf_gpu_get_stats",
-    "letkf_gpu_general_counts", "letkf_gpu_last_error", "letkf_gpu_destroy", "letkf_gpu_launch_count",
+    "letkf_gpu_general_counts", "letkf_gpu_set_scratch_limit", "letkf_gpu_last_error", "letkf_gpu_destroy", "letkf_gpu_launch_count",
     "letkf_gpu_core_batch_noalloc", "letkf_decomp_dims", "letkf_gpu_autotune",
     "letkf_batch_create", "letkf_batch_launch", "letkf_batch_sync", "letkf_batch_launches",
     "letkf_batch_destroy", "letkf_gpu_set_list_limit", "letkf_gpu_set_cube_range", "letkf_gpu_run_members",
@@ -151,6 +151,7 @@ def load_library(path: str = LIB_PATH):
     L.letkf_batch_launches.restype = i64
     L.letkf_batch_destroy.argtypes = [vp]
     L.letkf_gpu_set_list_limit.argtypes = [vp, i64]
+    L.letkf_gpu_set_scratch_limit.argtypes = [vp, i64]
     L.letkf_gpu_set_cube_range.argtypes = [vp, i64, i64]
     L.letkf_gpu_run_members.argtypes = [vp, vp, C.POINTER(Obs), C.POINTER(Blend), vp, vp, vp, i32]
     L.letkf_gpu_obs_from_records.argtypes = [vp, i64, i32, i32, vp, vp, vp, vp, vp, vp, C.POINTER(Obs), i32]
@@ -357,6 +358,10 @@ class LetkfGPU:
         """Most local-list entries held at once (0: from free memory); runs
         whose lists exceed it go through consecutive cube windows."""
         self._check(self.L.letkf_gpu_set_list_limit(self.h, int(max_entries)), "set_list_limit")
+
+    def set_scratch_limit(self, nbytes: int = 0):
+        """Most bytes of the FP64 form's tensor-core intermediates (0: as many as fit)."""
+        self._check(self.L.letkf_gpu_set_scratch_limit(self.h, int(nbytes)), "set_scratch_limit")
 
     def set_wait_limit(self, polls: int = -1):
         """Most polls of each bounded tensor-core wait (< 0: the default; 0:

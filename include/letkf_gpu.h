@@ -283,6 +283,17 @@ int letkf_struct_endnn2atm_a(int n, int nx, int ny, int n_max, int n_start, cons
  * in the reference, whose ranks each hold their own sub-domain's lists.     */
 int letkf_gpu_set_list_limit(letkf_ctx *ctx, int64_t max_entries);
 
+/* Most bytes of device memory that the FP64 form's tensor-core path (ensembles
+ * of 32, 48, 64, 96 and 128) may hold for its intermediates in a run, and as
+ * many in the batched core; 0 (the default): as many as fit, up to about 2 GB.  It
+ * then takes the problems in smaller blocks, with the same results; where not
+ * even 1,024 problems (or the run's, if fewer) fit, the general FP64 kernel
+ * solves them (letkf_gpu_general_counts).  letkf_gpu_run_members splits the state
+ * only where the split state fits the limit, too.  Not for a context of a
+ * letkf_batch: a smaller limit gives buffers back that its graph uses.  No
+ * counterpart in the reference.                                              */
+int letkf_gpu_set_scratch_limit(letkf_ctx *ctx, int64_t bytes);
+
 /* Analyse only cubes first .. first+count-1 (count < 0: every cube), as one
  * DA rank analyses its own sub-domain (letkf_run's nx x ny arrays,
  * letkf.F90:169-176); cube = lat block + (lat blocks) * lon block, so with
