@@ -410,9 +410,8 @@ size_t list_entry_bytes(const letkf_ctx *ctx)
     return sizeof(int32_t) + sizeof(double) + (lg_is_mixed(ctx->params.precision) ? sizeof(float2) : 0);
 }
 
-// Entries the list pool may hold: the caller's limit, else the device's free
-// memory plus the pool's own, less the core's intermediates that are still to
-// be allocated and 1 GiB for the rest of the run.
+// Entries the list pool may hold: the caller's limit, else from the device's
+// free memory (lg_pool_entries).
 int64_t pool_limit(letkf_ctx *ctx)
 {
     if (ctx->list_limit > 0) return ctx->list_limit;
@@ -420,10 +419,10 @@ int64_t pool_limit(letkf_ctx *ctx)
     if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) return std::max<int64_t>(ctx->list_cap, 1);
     const size_t held = ctx->d_lidx.n * sizeof(int32_t) + ctx->d_lrloc.n * sizeof(double) +
                         ctx->d_lmeta.n * sizeof(float2);
-    const size_t keep = ((size_t)1 << 30) + (lg_is_mixed(ctx->params.precision) ? lg_wide_scratch_bytes(ctx)
-                                                                                 : lg_f64_scratch_bytes(ctx));
-    const size_t avail = fr + held > keep ? fr + held - keep : 0;
-    return std::max<int64_t>((int64_t)(avail / list_entry_bytes(ctx)), 1);
+    return lg_pool_entries((int64_t)fr, (int64_t)held,
+                           (int64_t)(lg_is_mixed(ctx->params.precision) ? lg_wide_scratch_bytes(ctx)
+                                                                        : lg_f64_scratch_bytes(ctx)),
+                           (int64_t)list_entry_bytes(ctx));
 }
 
 void release_pool(letkf_ctx *ctx)
@@ -648,6 +647,17 @@ void fill_stats(letkf_ctx *ctx, const unsigned long long *cnt)
 }
 
 }  // namespace
+
+// List entries of `entry` bytes that free_bytes of device memory and the pool's
+// own `held` bytes leave, less 1 GiB for the rest of the run and the core's
+// intermediates that are still to be allocated, which take at most half of the
+// rest: they go in smaller blocks where memory is short, while lists that do not
+// fit are searched window by window.
+extern "C" int64_t lg_pool_entries(int64_t free_bytes, int64_t held, int64_t scratch, int64_t entry)
+{
+    const int64_t room = std::max<int64_t>(free_bytes + held - ((int64_t)1 << 30), 0);
+    return std::max<int64_t>((room - std::min(scratch, room / 2)) / entry, 1);
+}
 
 void lg_count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 
