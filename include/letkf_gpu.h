@@ -44,7 +44,9 @@ extern "C" {
 #define LETKF_ERR_UNSUPPORTED   -6   /* configuration not supported              */
 #define LETKF_ERR_STATE         -7   /* call order (e.g. no run yet)             */
 
-/* letkf_gpu_run flags */
+/* letkf_gpu_run flags.  State arrays (xb, xa) in device memory start on 16-byte
+ * boundaries in the mixed forms; the FP64 form takes them on any double (between
+ * those boundaries with its general kernel).                                 */
 #define LETKF_HOST_PTRS    0   /* xb/axb/obs/xa/axa are host memory                */
 #define LETKF_DEVICE_PTRS  1   /* xb/axb/obs/xa/axa are device memory of this GPU */
 
@@ -217,8 +219,9 @@ typedef struct letkf_blend {
  * :214-258): xa_out [col][row][member] the analysis members, spread_b and
  * spread_a [col][row] the background and analysis spreads sqrt(sum d^2 / ens).
  * With one column per cube, no overlap and no vertical localization (and an
- * ensemble of at most 64 in the mixed forms) the split and the blend are done
- * inside the analysis (H reads the members, the update forms each row's mean
+ * ensemble of at most 64 in the mixed forms, or of less than 32 in the FP64
+ * form, whose tensor-core path takes the split state where it fits the device)
+ * the split and the blend are done inside the analysis (H reads the members, the update forms each row's mean
  * and writes the blended members and both spreads), so the call makes no
  * pass over the state beyond those of letkf_gpu_run; otherwise they are one
  * pass each before and after it.  Every cube is analysed (no cube range).
@@ -413,7 +416,10 @@ int letkf_gpu_set_schedule(letkf_ctx *ctx, int chunk);
  * status of the contexts (their stats are updated; a list pool too small for
  * new inputs shows as LETKF_ERR_ALLOC: create the batch again).  Contexts with
  * decomposed observation sets are not captured (LETKF_ERR_UNSUPPORTED).
- * Do not run a captured context by itself while its batch may be running.   */
+ * Do not run a captured context by itself while its batch may be running.  A
+ * later call of a captured context that needs larger buffers than the captured
+ * run (more observations, a wider cube range) moves them: create the batch
+ * again.  letkf_gpu_core_batch has buffers of its own.                       */
 typedef struct letkf_batch letkf_batch;
 int letkf_batch_create(letkf_batch **batch, int n, letkf_ctx *const *ctxs, const double *const *xb,
                        const double *const *axb, const letkf_obs *obs, double *const *xa,
