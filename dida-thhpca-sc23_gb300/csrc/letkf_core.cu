@@ -557,8 +557,8 @@ cudaError_t lg_launch_core_fp64(letkf_ctx *ctx, const LgGrid &g, const double *x
     src.olnp = (ctx->params.overlap == 0 && ctx->params.vert_dist > 0.0) ? ctx->d_olnp.p : nullptr;
     double *tr = keep_trans ? ctx->d_trans.p : nullptr, *w = keep_trans ? ctx->d_w.p : nullptr;
     // the FP64 pipe does two multiply-adds per clock and SM; the whole run, k =
-    // 64, 16,200 columns: 308 ms with k_core_fp64, 15.5 on the tensor cores; k = 32:
-    // 60.1 and 6.8; k = 96, 8,978 columns: 736 and 29.4.  Its update moves 16
+    // 64, 16,200 columns: 308 ms with k_core_fp64, 15.7 on the tensor cores; k = 32:
+    // 60.1 and 6.6; k = 96, 8,978 columns: 736 and 29.8.  Its update moves 16
     // bytes at a time: a caller's device arrays that start between those
     // boundaries stay with k_core_fp64
     if (lg_f64_supports(g.k) && !ctx->members_on && lg_aligned16(xb) && lg_aligned16(xa)) {

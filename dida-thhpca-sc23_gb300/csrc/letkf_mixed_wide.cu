@@ -14,14 +14,14 @@
 //   * the update's operands (xb rows and T, k members deep) are two
 //     128-byte-swizzled tiles along the member axis.
 // Three launches per block of cubes, as the narrow core's at k = 64: the A build
-// and the update on the tensor cores (a work queue, one CTA per SM), and
-// between them the eigenproblems (k_wide_eig), which spend their time on
+// and the update on the tensor cores (a work queue; one CTA per SM, the update
+// two at k = 96), and between them the eigenproblems (k_wide_eig), which spend their time on
 // shuffles, barriers and dependent arithmetic and therefore run several CTAs
 // per SM.  The FP32 Jacobi takes the hierarchical ordering over blocks of two
 // columns (k = 128, lg_jacobi32b2) or three (k = 96, lg_jacobi32b3).  One
 // launch with all stages, a cube at a time on 8 warps per SM, took 64.5 ms on
 // 28,800 cubes of k = 96 (72% of it in the Jacobi, a third of the issue slots
-// used); the three take 31.7 ms: 4.1 A build, 22.1 eigenproblems, 4.4 update.
+// used); the three take 29.2 ms: 3.7 A build, 22.1 eigenproblems, 3.4 update.
 #include <algorithm>
 
 #include "letkf_internal.cuh"
