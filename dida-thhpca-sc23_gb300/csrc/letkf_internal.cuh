@@ -557,6 +557,7 @@ cudaError_t lg_launch_core_mixed(letkf_ctx *ctx, const LgGrid &g, const double *
 // done = false when its intermediates do not fit the device's free memory.
 bool lg_f64_supports(int k);
 extern "C" int64_t lg_pool_entries(int64_t free_bytes, int64_t held, int64_t scratch, int64_t entry);
+extern "C" int lg_split_fits(int64_t room, int64_t split, int64_t nobs, int64_t k);
 inline bool lg_aligned16(const void *p) { return ((uintptr_t)p & 15) == 0; }
 cudaError_t lg_launch_core_f64(letkf_ctx *ctx, const LgGrid &g, const LgRowSrc &src, int64_t rows,
                                const int64_t *loff, const int32_t *lcnt, int64_t cube0, int64_t cube1,

@@ -168,7 +168,37 @@ unsigned grid_for(int64_t nrows, int per)
     return (unsigned)(want < (1 << 20) ? want : (1 << 20));
 }
 
+// Room for the split state, as far as it is not held yet.
+bool split_has_room(letkf_ctx *ctx, size_t nstate, size_t nmean, int64_t nobs)
+{
+    size_t grow = 0, held = 0, fr = 0, tot = 0;
+    auto add = [&](const DevBuf<double> &b, size_t n) {
+        if (n <= b.n) return;
+        grow += n * sizeof(double);
+        held += b.n * sizeof(double);
+    };
+    add(ctx->d_xb, nstate);
+    add(ctx->d_xa, nstate);
+    add(ctx->d_axb, nmean);
+    add(ctx->d_axa, nmean);
+    if (grow == 0) return true;
+    if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return lg_split_fits((int64_t)(fr + held), (int64_t)grow, nobs, ctx->k) != 0;
+}
+
 }  // namespace
+
+// Whether `room` bytes hold `split` bytes of split state and what the run cannot do
+// without beside it: the observations' arrays (y in k doubles, and up to 128 bytes) and
+// 2 GiB, of which the list pool leaves 1 GiB and the rest serves it and the
+// core's intermediates (both go in smaller pieces where memory is short).
+extern "C" int lg_split_fits(int64_t room, int64_t split, int64_t nobs, int64_t k)
+{
+    return split + nobs * (8 * k + 128) + ((int64_t)2 << 30) <= room;
+}
 
 extern "C" int letkf_gpu_run_members(letkf_ctx *ctx, const double *xb_in, const letkf_obs *obs,
                                      const letkf_blend *blend, double *xa_out, double *spread_b,
@@ -207,10 +237,11 @@ extern "C" int letkf_gpu_run_members(letkf_ctx *ctx, const double *xb_in, const 
     // The FP64 form's tensor-core path (letkf_f64.cu) takes the split state:
     // its analysis with two passes over the state is far shorter than the
     // fused k_core_fp64 (4 degrees, k = 64, 4,050 columns: 4.9 against 81 ms
-    // on the device).  Where the split state does not fit the device, or the
-    // context's limit, the fused form stays.
+    // on the device).  Where the split state does not fit the device beside the
+    // rest of the run, or the context's limit, the fused form stays.
     if (fused && !lg_is_mixed(ctx->params.precision) && lg_f64_supports(k) &&
-        (ctx->scratch_limit == 0 || 16 * (nstate + nmean) <= (size_t)ctx->scratch_limit)) {
+        (ctx->scratch_limit == 0 || 16 * (nstate + nmean) <= (size_t)ctx->scratch_limit) &&
+        split_has_room(ctx, nstate, nmean, obs->nobs)) {
         cudaError_t e = ctx->d_xb.reserve(nstate);
         if (e == cudaSuccess) e = ctx->d_axb.reserve(nmean);
         if (e == cudaSuccess) e = ctx->d_xa.reserve(nstate);
